@@ -1,6 +1,8 @@
 // GPTQ / AWQ -> Marlin tile layout repacking.
 //
-// One thread block owns a strip of TK quantised rows (16, or 32 for the 8-bit-activation
+// 16-bit-activation layouts in checkpoint row order take RepackWarpKernel: a warp turns 64 columns by 16 k
+// at a time in registers.  8-bit-activation layouts and activation-order checkpoints (each output word
+// then gathers from arbitrary rows) take RepackKernel: one thread block owns a strip of TK quantised rows (16, or 32 for the 8-bit-activation
 // layouts) by up to 256 columns.  It first expands that strip from the source packing into
 // an unpacked byte tile in shared memory with coalesced word loads, then every thread
 // assembles four consecutive output words from the tile and writes them with one 16-byte
@@ -118,6 +120,180 @@ RepackKernel(const uint32_t* __restrict__ in, const int32_t* __restrict__ perm,
   }
 }
 
+// ---- one warp per 64-column chunk, no shared memory -----------------------------------------------
+//
+// Lane 4 g + c of a chunk owns the output words of columns 16 t + g and 16 t + g + 8 (t = 0..3) for rows
+// 2c, 2c + 1, 2c + 8, 2c + 9: contiguous, and stored by 16-byte writes that cover 512 (1024) contiguous
+// bytes per warp.  The words it needs come straight from global memory in whole 32-byte sectors; bytes and
+// nibbles are moved a word at a time, where the staged form above handles every element by itself in
+// shared memory.  kUnroll k-tiles per warp keep that many tiles' loads in flight.
+constexpr int kUnroll = 4;
+
+// x = four bytes (one per source) -> low nibbles in bits 0..15, high nibbles in bits 16..31.
+__device__ __forceinline__ uint32_t SplitNibbles(uint32_t x) {
+  const uint32_t lo = x & 0x0F0F0F0Fu, hi = (x >> 4) & 0x0F0F0F0Fu;
+  return __byte_perm(lo | (lo >> 4), hi | (hi >> 4), 0x6420u);
+}
+
+template <int kBits, Source kSource>
+struct WarpTile;
+
+// A source word holds rows 8r .. 8r + 7 of one column.  Lane (g, c) loads the four words of columns
+// 16 c + g and + 8; the output words of its own (g, c) take byte c of the four words of each t, so the four
+// lanes of a g exchange a 4 x 4 table of words.
+template <>
+struct WarpTile<4, Source::kGptq> {
+  uint32_t w[4];
+  __device__ __forceinline__ void Load(const uint32_t* in, int kt, int size_n, int n0, int lane) {
+    const uint32_t* src = in + static_cast<int64_t>(2 * kt) * size_n + n0 + 16 * (lane & 3) + (lane >> 2);
+    w[0] = __ldg(src);
+    w[1] = __ldg(src + size_n);
+    w[2] = __ldg(src + 8);
+    w[3] = __ldg(src + size_n + 8);
+  }
+  __device__ __forceinline__ void Store(uint32_t* out, int lane) const {
+    // byte b of the four words side by side, for b = 0..3
+    const uint32_t p0 = __byte_perm(w[0], w[1], 0x5140u), p1 = __byte_perm(w[2], w[3], 0x5140u);
+    const uint32_t p2 = __byte_perm(w[0], w[1], 0x7362u), p3 = __byte_perm(w[2], w[3], 0x7362u);
+    uint32_t m[4] = {SplitNibbles(__byte_perm(p0, p1, 0x5410u)), SplitNibbles(__byte_perm(p0, p1, 0x7632u)),
+                     SplitNibbles(__byte_perm(p2, p3, 0x5410u)), SplitNibbles(__byte_perm(p2, p3, 0x7632u))};
+    // lane t of the quad holds column m[c] of t; transpose, so that lane c holds its words of t = 0..3
+    const bool odd = lane & 1, upper = lane & 2;
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? m[i] : m[i + 1], 1);
+      if (odd) {
+        m[i] = got;
+      } else {
+        m[i + 1] = got;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, upper ? m[i] : m[i + 2], 2);
+      if (upper) {
+        m[i] = got;
+      } else {
+        m[i + 2] = got;
+      }
+    }
+    reinterpret_cast<uint4*>(out)[lane] = make_uint4(m[0], m[1], m[2], m[3]);
+  }
+};
+
+// A source word holds rows 4r .. 4r + 3 of one column: an output word is two bytes of each of two words.
+template <>
+struct WarpTile<8, Source::kGptq> {
+  uint32_t w[16];
+  __device__ __forceinline__ void Load(const uint32_t* in, int kt, int size_n, int n0, int lane) {
+    const uint32_t* src = in + static_cast<int64_t>(4 * kt + ((lane & 3) >> 1)) * size_n + n0 + (lane >> 2);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      w[2 * j] = __ldg(src + 8 * j);
+      w[2 * j + 1] = __ldg(src + 2 * static_cast<int64_t>(size_n) + 8 * j);
+    }
+  }
+  __device__ __forceinline__ void Store(uint32_t* out, int lane) const {
+    const uint32_t select = (lane & 1) ? 0x7362u : 0x5140u;
+    uint32_t m[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[j] = __byte_perm(w[2 * j], w[2 * j + 1], select);
+    reinterpret_cast<uint4*>(out)[2 * lane] = make_uint4(m[0], m[1], m[2], m[3]);
+    reinterpret_cast<uint4*>(out)[2 * lane + 1] = make_uint4(m[4], m[5], m[6], m[7]);
+  }
+};
+
+// A source word holds eight columns of one row, column j in nibble {0, 4, 1, 5, 2, 6, 3, 7}[j].  Word 2t + h
+// of a row has columns 16 t + 8 h + 0..7: the lane takes the nibble of its g from four rows' words.
+template <>
+struct WarpTile<4, Source::kAwq> {
+  uint4 w[8];
+  __device__ __forceinline__ void Load(const uint32_t* in, int kt, int size_n, int n0, int lane) {
+    const int64_t pitch = size_n / 8;
+    const uint32_t* src = in + (static_cast<int64_t>(kt) * 16 + 2 * (lane & 3)) * pitch + n0 / 8;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint4* row = reinterpret_cast<const uint4*>(src + ((r & 1) + 8 * (r >> 1)) * pitch);
+      w[2 * r] = __ldg(row);
+      w[2 * r + 1] = __ldg(row + 1);
+    }
+  }
+  __device__ __forceinline__ void Store(uint32_t* out, int lane) const {
+    const int g = lane >> 2;
+    const int shift = 4 * ((g >> 1) + 4 * (g & 1));
+    uint32_t m[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      uint32_t v[4][2];  // rows 2c, 2c + 1, 2c + 8, 2c + 9; columns g, g + 8
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint4& q = w[2 * r + (t >> 1)];
+        v[r][0] = ((t & 1) ? q.z : q.x) >> shift;
+        v[r][1] = ((t & 1) ? q.w : q.y) >> shift;
+      }
+      m[t] = (v[0][0] & 0xFu) | ((v[2][0] & 0xFu) << 4) | ((v[0][1] & 0xFu) << 8) | ((v[2][1] & 0xFu) << 12) |
+             ((v[1][0] & 0xFu) << 16) | ((v[3][0] & 0xFu) << 20) | ((v[1][1] & 0xFu) << 24) | (v[3][1] << 28);
+    }
+    reinterpret_cast<uint4*>(out)[lane] = make_uint4(m[0], m[1], m[2], m[3]);
+  }
+};
+
+// A source word holds four columns of one row, column j in byte {0, 2, 1, 3}[j].
+template <>
+struct WarpTile<8, Source::kAwq> {
+  uint32_t w[32];
+  __device__ __forceinline__ void Load(const uint32_t* in, int kt, int size_n, int n0, int lane) {
+    const int64_t pitch = size_n / 4;
+    const uint32_t* src = in + (static_cast<int64_t>(kt) * 16 + 2 * (lane & 3)) * pitch + n0 / 4 + (lane >> 4);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[8 * r + j] = __ldg(src + ((r & 1) + 8 * (r >> 1)) * pitch + 2 * j);
+    }
+  }
+  __device__ __forceinline__ void Store(uint32_t* out, int lane) const {
+    const int j4 = (lane >> 2) & 3, byte = ((j4 & 1) << 1) | (j4 >> 1);
+    const uint32_t select = static_cast<uint32_t>(byte) | (static_cast<uint32_t>(byte + 4) << 4);
+    uint32_t m[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      m[j] = __byte_perm(__byte_perm(w[j], w[16 + j], select), __byte_perm(w[8 + j], w[24 + j], select), 0x5410u);
+    }
+    reinterpret_cast<uint4*>(out)[2 * lane] = make_uint4(m[0], m[1], m[2], m[3]);
+    reinterpret_cast<uint4*>(out)[2 * lane + 1] = make_uint4(m[4], m[5], m[6], m[7]);
+  }
+};
+
+template <int kBits, Source kSource>
+__global__ void __launch_bounds__(kThreads) RepackWarpKernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                            int size_k, int size_n) {
+  constexpr int kU = kBits == 8 && kSource == Source::kAwq ? 1 : kBits == 8 || kSource == Source::kAwq ? 2 : kUnroll;
+  const int lane = threadIdx.x & 31, chunks = size_n / 64, tiles = size_k / 16;
+  const long long unit = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
+  const int kt0 = static_cast<int>(unit / chunks) * kU, chunk = static_cast<int>(unit % chunks);
+  WarpTile<kBits, kSource> tile[kU];
+#pragma unroll
+  for (int u = 0; u < kU; ++u) {
+    if (kt0 + u < tiles) tile[u].Load(in, kt0 + u, size_n, chunk * 64, lane);
+  }
+  constexpr int kWords = 1024 * kBits / 32;  // output words of a tile
+#pragma unroll
+  for (int u = 0; u < kU; ++u) {
+    if (kt0 + u < tiles) tile[u].Store(out + (static_cast<int64_t>(kt0 + u) * chunks + chunk) * kWords, lane);
+  }
+}
+
+template <int kBits, Source kSource>
+int LaunchWarps(const int32_t* in, int32_t* out, int64_t size_k, int64_t size_n, cudaStream_t stream) {
+  constexpr int kU = kBits == 8 && kSource == Source::kAwq ? 1 : kBits == 8 || kSource == Source::kAwq ? 2 : kUnroll;
+  const int64_t units = (size_n / 64) * ((size_k / 16 + kU - 1) / kU);
+  const int64_t blocks = (units + kThreads / 32 - 1) / (kThreads / 32);
+  RepackWarpKernel<kBits, kSource><<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(
+      reinterpret_cast<const uint32_t*>(in), reinterpret_cast<uint32_t*>(out), static_cast<int>(size_k),
+      static_cast<int>(size_n));
+  return CheckLaunch("marlin repack launch");
+}
+
 template <int kBits, bool kA8, Source kSource>
 int Launch(const int32_t* in, const int32_t* perm, int32_t* out, int64_t size_k, int64_t size_n,
            cudaStream_t stream) {
@@ -162,10 +338,10 @@ extern "C" int infiniops_b200_gptq_marlin_repack(const int32_t* b_q_weight, cons
   }
   if (num_bits == 4) {
     return is_a_8bit ? Launch<4, true, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s)
-                     : Launch<4, false, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s);
+                     : LaunchWarps<4, Source::kGptq>(b_q_weight, out, size_k, size_n, s);
   }
   return is_a_8bit ? Launch<8, true, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s)
-                   : Launch<8, false, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s);
+                   : LaunchWarps<8, Source::kGptq>(b_q_weight, out, size_k, size_n, s);
 }
 
 extern "C" int infiniops_b200_awq_marlin_repack(const int32_t* b_q_weight, int64_t size_k,
@@ -175,9 +351,12 @@ extern "C" int infiniops_b200_awq_marlin_repack(const int32_t* b_q_weight, int64
   if (const int rc = CheckCommon(b_q_weight, out, size_k, size_n, num_bits, is_a_8bit)) return rc;
   auto s = static_cast<cudaStream_t>(stream);
   if (num_bits == 4) {
-    return is_a_8bit ? Launch<4, true, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s)
-                     : Launch<4, false, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
+    if (is_a_8bit) return Launch<4, true, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
+    // (the warp kernel reads AWQ rows by 16-byte loads; `b_q_weight` itself may sit on any word)
+    return reinterpret_cast<uintptr_t>(b_q_weight) % 16 == 0
+               ? LaunchWarps<4, Source::kAwq>(b_q_weight, out, size_k, size_n, s)
+               : Launch<4, false, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
   }
   return is_a_8bit ? Launch<8, true, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s)
-                   : Launch<8, false, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
+                   : LaunchWarps<8, Source::kAwq>(b_q_weight, out, size_k, size_n, s);
 }
