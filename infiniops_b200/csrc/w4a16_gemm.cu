@@ -38,6 +38,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "w4a16_few_rows.cuh"
 
 namespace iob {
 namespace {
@@ -2494,6 +2495,31 @@ void FillDense(const iob_gemm_problem& g, unsigned char* scratch, const ScratchP
   SetGroupMap(p);
 }
 
+FewRowsWeights FewRowsWeightsOf(int64_t b_type_id) {
+  return BitsOf(b_type_id) == 4 ? FewRowsWeights::kInt4
+         : b_type_id == IOB_QTYPE_FLOAT8_E4M3FN ? FewRowsWeights::kFloat8 : FewRowsWeights::kInt8;
+}
+
+// The same problem for the kernel without tensor memory; `p` has its placement.
+FewRowsParams FewRowsOf(const iob_gemm_problem& g, const GemmParams& p, const void* activations) {
+  FewRowsParams f{};
+  f.a = activations;
+  f.wq = reinterpret_cast<const uint32_t*>(g.b_q_weight);
+  f.scales = g.b_scales;
+  f.zeros = reinterpret_cast<const uint32_t*>(g.b_zeros);
+  f.bias = g.b_bias;
+  f.out = g.out;
+  f.m = static_cast<int>(g.size_m);
+  f.n = static_cast<int>(g.size_n);
+  f.k = static_cast<int>(g.size_k);
+  f.groups = static_cast<int>(g.num_groups);
+  f.group_size = static_cast<int>(g.size_k / g.num_groups);
+  f.layout = p.layout;
+  f.out_ld = p.out_ld;
+  f.out_col0 = p.out_col0;
+  return f;
+}
+
 }  // namespace
 }  // namespace iob
 
@@ -2546,6 +2572,12 @@ extern "C" int infiniops_b200_marlin_gemm_placed(const iob_gemm_problem* problem
     }
     if (const int rc = CheckLaunch("marlin_gemm column permutation launch")) return rc;
     activations = base + plan.gathered_off;
+  }
+  // Up to 16 rows: the register-operand kernel (no peers to write, no completion signal to give).  The four
+  // linears of a 4096 / 14336 layer, a launch each: 74.9 -> 68.5 us at 1 row (uint4), 73.5 -> 61.7 at 16
+  // (uint4b8, float16), 121.5 -> 64.3 at 7 (8-bit).  The line lies at its second token tile of 8.
+  if (g.size_m <= kFewRows && g.n_peers == 0 && signal == nullptr) {
+    return FewRowsGemm(a_dtype, FewRowsWeightsOf(b_type_id), FewRowsOf(g, p, activations), static_cast<cudaStream_t>(stream));
   }
   // Prefill-sized problems whose columns pair up run two blocks per 256 x 256 output tile.
   const bool pair = tok == 256 && g.size_n % (2 * kTileN) == 0 && NumSms() >= 2;
@@ -2733,6 +2765,13 @@ extern "C" int infiniops_b200_moe_wna16_marlin_gemm_ex(
   const void* gathered = a_sorted && perm == nullptr ? a : base + plan.gathered_off;
   const int out_rows = static_cast<int>(size_m * top_k);
   const int gather_grid = static_cast<int>(std::min<int64_t>(sorted_cap, 4 * NumSms()));
+  // Routing blocks of up to 16 rows: the register-operand kernel, which reads the tokens' rows where they are
+  // unless the gather has something else to do (column order, by-products); no scatter, no completion signal.
+  // One token over 8 experts of 4096 / 14336: 109 -> 94 us for the whole chain; 16 tokens over 256 of 7168 / 2048,
+  // top 8: 820 -> 787 us.
+  const bool few_rows = moe_block_size <= kFewRows && (options == nullptr || (options->row_dest == nullptr && options->signal == nullptr)) &&
+                        blocks * (size_n / 64) <= (1 << 24);
+  const bool gathers = perm != nullptr || (!a_sorted && !(few_rows && position == nullptr && block_rows_out == nullptr));
   if (position != nullptr &&
       cudaMemsetAsync(position, 0xFF, static_cast<size_t>(out_rows) * sizeof(int32_t), s) != cudaSuccess) {
     return Fail(IOB_CUDA_ERROR, "%s: could not clear `route_position`", op);
@@ -2751,8 +2790,8 @@ extern "C" int infiniops_b200_moe_wna16_marlin_gemm_ex(
     } else {
       launch(static_cast<__half*>(nullptr));
     }
-  } else if (a_sorted) {
-    // `a` already holds one row per sorted position: nothing to gather
+  } else if (!gathers) {
+    // `a` already holds one row per sorted position, or its rows are read where they are
   } else if (a_dtype == IOB_BF16) {
     GatherRowsKernel<__nv_bfloat16><<<gather_grid, 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(a), reinterpret_cast<__nv_bfloat16*>(base + plan.gathered_off), sorted_token_ids,
@@ -2830,6 +2869,35 @@ extern "C" int infiniops_b200_moe_wna16_marlin_gemm_ex(
       }
     }
     if (const int rc = SetSignal(op, options->signal, p)) return rc;
+  }
+  if (few_rows) {
+    FewRowsParams f{};
+    f.a = gathers ? gathered : a;
+    f.wq = p.wq;
+    f.scales = p.scales;
+    f.zeros = p.zeros;
+    f.bias = p.bias;
+    f.out = p.out;
+    f.m = p.m;
+    f.n = p.n;
+    f.k = p.k;
+    f.groups = p.groups;
+    f.group_size = p.group_size;
+    f.layout = p.layout;
+    f.out_ld = p.fuse_silu ? p.n / 2 : p.n;
+    f.sorted_ids = p.sorted_ids;
+    f.expert_ids = p.expert_ids;
+    f.num_post_pad = p.num_post_pad;
+    f.topk_weights = p.topk_weights;
+    f.top_k = p.top_k;
+    f.block_size = p.block_size;
+    f.mul_weights = p.mul_weights;
+    f.out_rows = p.out_rows;
+    f.a_sorted = a_sorted || gathers ? 1 : 0;
+    f.out_sorted = p.out_sorted;
+    f.blocks = static_cast<int>(blocks);
+    f.fuse_silu = p.fuse_silu;
+    return FewRowsGemm(a_dtype, FewRowsWeightsOf(b_type_id), f, s);
   }
   CUtensorMap c_map = w_map;  // unused while rows are scattered
   if (p.out_sorted) {
