@@ -761,8 +761,11 @@ __device__ __forceinline__ void GemmBody(const Problem* probs, int count) {
   constexpr int kActStages = Sh::kActStages;
   static_assert(kStage <= StageBytes(kTok, kBits), "stage layout");
   // The lanes of a pass wait for each other, so a pass must stay well below the ring size or the
-  // ring would drain between passes.
-  constexpr int kProdLanes = kStages >= 8 ? 4 : kStages >= 4 ? 2 : 1;
+  // ring would drain between passes.  And a ring slot must always meet the same lane: the sets free
+  // their slots independently of one another, so a lane that meets a slot for the first time can be two
+  // phases ahead of its barrier, where the one parity bit reads "free" while the slot is still in use.
+  constexpr int kProdLanes = kStages % 4 == 0 && kStages >= 8 ? 4 : kStages % 3 == 0 && kStages >= 9 ? 3 : kStages >= 4 ? 2 : 1;
+  static_assert(kStages % kProdLanes == 0, "a ring slot must always meet the same producer lane");
   constexpr int kTmemCols = kPair ? 512 : TmemColsFor(kTok);
   constexpr int kDequantWarps = 4 * kSets;
   constexpr int kIssuerWarps = IssuersFor(kTok);        // warps reserved for issuing

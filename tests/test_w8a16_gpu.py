@@ -189,3 +189,30 @@ def test_routed_gemm_with_8bit_weights_and_zero_points():
             ref[t * top_k + j] = (x[t].float() @ oq.dequantize(qs[e], ss[e], zs[e], 8)) * tw[t * top_k + j]
     assert not torch.isnan(out.float()).any()
     assert rel_max_err(out, ref) <= TOL
+
+
+@pytest.mark.parametrize("m", (17, 32))
+def test_8bit_ring_wraps_on_cold_weights(m):
+    """The 9-slot ring of the 8-bit tiles of up to 32 rows, wrapped many times at the pace of memory (float16, weights
+    larger than the caches, launches back to back): every launch gives the bits of the first, and those are right.
+    A slot that met two producer lanes could be refilled while its weights were still being read.
+
+    Tolerance: weights rounded once to float16 and the product once (2^-11 each), sums in fp32."""
+    from infiniops_b200 import capi
+
+    k, base, times, dtype = 4096, 512, 56, torch.float16
+    q, scales, marlin = _weights(k, base, 128, dtype, 8200)
+    n = base * times
+    words = [marlin.repeat(1, times) for _ in range(3)]
+    a = torch.randn((m, k), generator=torch.Generator().manual_seed(m)).to(dtype)
+    x, s = a.cuda(), scales.cuda().repeat(1, times)
+    first = torch.empty((m, n), dtype=dtype, device="cuda")
+    capi.marlin_gemm(x, words[0], None, s, None, UINT8B128, m, n, k, first)
+    outs = [torch.empty_like(first) for _ in range(30)]
+    for i, out in enumerate(outs):
+        capi.marlin_gemm(x, words[i % 3], None, s, None, UINT8B128, m, n, k, out)
+    torch.cuda.synchronize()
+    assert capi.scratch_status(capi.scratch("cuda", 0)) == 0
+    assert all(torch.equal(out, first) for out in outs)
+    ref = (a.float() @ oq.dequantize(q, scales, None, 8)).repeat(1, times)
+    assert rel_max_err(first, ref) <= 2.0 ** -10
