@@ -213,7 +213,7 @@ __device__ __forceinline__ void FewRowsTile(const FewRowsParams& p, int tile, in
     if (expert < 0) return;
   }
 
-  // ---- weights under way (constants of the model: not waited for) -------------------------------
+  // ---- weights under way ------------------------------------------------------------------------
   const int words_per_row = p.n * (kW == FewRowsWeights::kInt4 ? 2 : 4);
   const uint32_t* wq = p.wq + static_cast<size_t>(expert) * (p.k / 16) * words_per_row +
                        n0 * (kW == FewRowsWeights::kInt4 ? 2 : 4) + lane * (kW == FewRowsWeights::kInt4 ? 4 : 8);
@@ -225,6 +225,31 @@ __device__ __forceinline__ void FewRowsTile(const FewRowsParams& p, int tile, in
     if constexpr (Words<kW>::kVecs == 2) CopyAsync16(slots + slot * kSlab + 16, next + 16);
     next += row_bytes;
   };
+  // Rows of the activations and of the result.  (Activation rows that are not live are never staged: whatever the
+  // buffers hold there reaches only its own columns of the products, which are not stored.)
+  auto set_rows = [&]() {
+    if constexpr (kMoe) {
+      if (tid < kRows) {
+        const int at = block * p.block_size + tid;
+        const int id = tid < p.block_size ? p.sorted_ids[at] : p.out_rows;
+        const bool live = id < p.out_rows;
+        row_in[tid] = live ? (p.a_sorted ? at : id / p.top_k) : -1;
+        // (sorted output: a block's padding rows are written too, as products of zeros)
+        row_out[tid] = p.out_sorted ? (tid < p.block_size ? at : -1) : live ? id : -1;
+      }
+    } else if (tid < kRows) {
+      row_in[tid] = row_out[tid] = tid < p.m ? tid : -1;
+    }
+    __syncthreads();
+  };
+  if constexpr (!kMoe) {
+    // Nothing that a predecessor in the stream could have written is read before the wait: not the activations, and
+    // not the weights, after a repack or an update.  (Weight copies ahead of it would give 0.2 to 1 us a launch:
+    // 4096 x 28672, 1 row, back to back 20.3 us against 21.2 with 4-bit weights, 26.8 against 28.5 with 8-bit ones.
+    // Pulling the slabs into L2 instead gives nothing: 21.2 to 21.5 us and 28.9 to 29.3.)
+    set_rows();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
   if (first < last) {
 #pragma unroll
     for (int s = 0; s < kRing; ++s) load(s);
@@ -233,23 +258,9 @@ __device__ __forceinline__ void FewRowsTile(const FewRowsParams& p, int tile, in
   if constexpr (kRing == kSteps) next += skip_bytes;
   CopyCommit();
 
-  // ---- rows --------------------------------------------------------------------------------------
-  if constexpr (kMoe) {
-    if (tid < kRows) {
-      const int at = block * p.block_size + tid;
-      const int id = tid < p.block_size ? p.sorted_ids[at] : p.out_rows;
-      const bool live = id < p.out_rows;
-      row_in[tid] = live ? (p.a_sorted ? at : id / p.top_k) : -1;
-      // (sorted output: a block's padding rows are written too, as products of zeros)
-      row_out[tid] = p.out_sorted ? (tid < p.block_size ? at : -1) : live ? id : -1;
-    }
-  } else if (tid < kRows) {
-    row_in[tid] = row_out[tid] = tid < p.m ? tid : -1;
-  }
-  // (Activation rows that are not live are never staged: whatever the buffers hold there reaches only its own
-  // columns of the products, which are not stored.)
-  __syncthreads();
-  // activations: a lane copies one 16-byte column piece of every second row
+  // ---- activations -------------------------------------------------------------------------------
+  if constexpr (kMoe) set_rows();
+  // a lane copies one 16-byte column piece of every second row
   const uint32_t act0 = Smem(smem) + warp * 2 * kActBytes;
   const unsigned char* a = static_cast<const unsigned char*>(p.a) + (lane & 15) * 16;
   const size_t a_row = static_cast<size_t>(p.k) * 2;
@@ -286,7 +297,6 @@ __device__ __forceinline__ void FewRowsTile(const FewRowsParams& p, int tile, in
     }
     CopyCommit();
   };
-  if constexpr (!kMoe) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (first < last) stage(first, 0);
 
   // ---- main loop ---------------------------------------------------------------------------------

@@ -901,7 +901,10 @@ __device__ __forceinline__ void GemmBody(const Problem* probs, int count) {
   };
 
   // From here on global memory is read and written: everything before was on-chip set-up.
-  // (The producer warp waits later: its first ring of weight copies does not depend on the predecessor.)
+  // That goes for the weights as well: a predecessor in the stream may have written them (a repack, an
+  // update).  Copying the first ring of weights ahead of the wait was no faster either: 32 rows of 4096 x 6144
+  // 16.0 us that way and 15.6 us so, 64 rows of 4096 x 28672 with 8-bit weights 80.5 and 74.9 us (back to back).
+  // (The producer warp finds its first stages before it waits.)
   if constexpr (!kMoe) {
     if (warp != 0) GridDependencyWait();
   }
@@ -920,8 +923,6 @@ __device__ __forceinline__ void GemmBody(const Problem* probs, int count) {
       Cursor c{make_walker(), Segment{}, static_cast<uint32_t>(lane), 0u, 0, 0};
       bool active = Locate<kMoe, kBatch>(c, cur->p.expert_ids);
       const int grp_rows = cur->p.group_size == 64 ? 2 : 1;
-      // The copies of one stage.  Packed weights, scales and zero points are constants of the model;
-      // only the activations can be the output of the kernel before this one.
       auto request_weights = [&](const Cursor& at) {
         [[maybe_unused]] const Problem* cur = kBatch ? probs + at.seg.prob : probs;
         const int s = at.it % kStages;
@@ -961,24 +962,7 @@ __device__ __forceinline__ void GemmBody(const Problem* probs, int count) {
           TmaLoad3D(stages_addr + s * kStage, &cur->a_map, 0, row0, 2 * at.Ks(), SmemAddr(&sh.full[s]));
         }
       };
-      if constexpr (!kMoe) {
-        // First trip round the ring (every slot is free): the weight copies go out before this
-        // kernel waits for its predecessor, so they overlap that kernel's tail; the activation
-        // copies follow once the predecessor's output is visible.
-        Cursor ahead = c;
-        bool ahead_active = active;
-        while (ahead_active && ahead.it < static_cast<uint32_t>(kStages)) {
-          request_weights(ahead);
-          ahead.it += kProdLanes;
-          ahead_active = Locate<kMoe, kBatch>(ahead, cur->p.expert_ids);
-        }
-        GridDependencyWait();
-        while (active && c.it < static_cast<uint32_t>(kStages)) {
-          request_activations(c);
-          c.it += kProdLanes;
-          active = Locate<kMoe, kBatch>(c, cur->p.expert_ids);
-        }
-      }
+      if constexpr (!kMoe) GridDependencyWait();
       uint32_t idle = 0;
       while (__any_sync(kMask, active)) {
         bool progressed = false;
