@@ -1,11 +1,11 @@
 // GPTQ / AWQ -> Marlin tile layout repacking.
 //
-// 16-bit-activation layouts in checkpoint row order take RepackWarpKernel: a warp turns 64 columns by 16 k
-// at a time in registers.  8-bit-activation layouts and activation-order checkpoints (each output word
-// then gathers from arbitrary rows) take RepackKernel: one thread block owns a strip of TK quantised rows (16, or 32 for the 8-bit-activation
-// layouts) by up to 256 columns.  It first expands that strip from the source packing into
-// an unpacked byte tile in shared memory with coalesced word loads, then every thread
-// assembles four consecutive output words from the tile and writes them with one 16-byte
+// GPTQ and 8-bit AWQ sources in checkpoint row order, for 16-bit activations, take RepackWarpKernel: a warp turns
+// 64 columns by 16 k at a time in registers.  4-bit AWQ sources, 8-bit-activation layouts and activation-order
+// checkpoints (each output word then gathers from arbitrary rows) take RepackKernel: one thread block owns a strip
+// of TK quantised rows (16, or 32 for the 8-bit-activation layouts) by up to 256 columns.  It first expands that
+// strip from the source packing into an unpacked byte tile in shared memory with coalesced word loads, then every
+// thread assembles four consecutive output words from the tile and writes them with one 16-byte
 // store.  The strip maps to one contiguous range of the output, so global traffic is one
 // coalesced read and one coalesced write of the weights.
 #include "common.cuh"
@@ -126,7 +126,12 @@ RepackKernel(const uint32_t* __restrict__ in, const int32_t* __restrict__ perm,
 // 2c, 2c + 1, 2c + 8, 2c + 9: contiguous, and stored by 16-byte writes that cover 512 (1024) contiguous
 // bytes per warp.  The words it needs come straight from global memory in whole 32-byte sectors; bytes and
 // nibbles are moved a word at a time, where the staged form above handles every element by itself in
-// shared memory.  kUnroll k-tiles per warp keep that many tiles' loads in flight.
+// shared memory.  Several k-tiles per warp keep more loads in flight (8-bit AWQ: one tile of 32 words).
+//
+// 4096 x 28672, cold, staged form -> this one: GPTQ 4-bit 50.2 -> 21.8 us (5.4 TB/s read plus written), GPTQ 8-bit
+// 80.6 -> 46.8, AWQ 8-bit 77.1 -> 64.2; 4096 x 4096 9.2 -> 5.4, 14.6 -> 9.5, 14.1 -> 11.9.  Not for 4-bit AWQ, whose
+// words hold eight columns of a row: eight lanes then load the same words for one nibble of each, 55.9 us staged
+// and 57.9 this way (2.6 and 3.5 at 1024 x 1024).
 constexpr int kUnroll = 4;
 
 // x = four bytes (one per source) -> low nibbles in bits 0..15, high nibbles in bits 16..31.
@@ -200,41 +205,6 @@ struct WarpTile<8, Source::kGptq> {
     for (int j = 0; j < 8; ++j) m[j] = __byte_perm(w[2 * j], w[2 * j + 1], select);
     reinterpret_cast<uint4*>(out)[2 * lane] = make_uint4(m[0], m[1], m[2], m[3]);
     reinterpret_cast<uint4*>(out)[2 * lane + 1] = make_uint4(m[4], m[5], m[6], m[7]);
-  }
-};
-
-// A source word holds eight columns of one row, column j in nibble {0, 4, 1, 5, 2, 6, 3, 7}[j].  Word 2t + h
-// of a row has columns 16 t + 8 h + 0..7: the lane takes the nibble of its g from four rows' words.
-template <>
-struct WarpTile<4, Source::kAwq> {
-  uint4 w[8];
-  __device__ __forceinline__ void Load(const uint32_t* in, int kt, int size_n, int n0, int lane) {
-    const int64_t pitch = size_n / 8;
-    const uint32_t* src = in + (static_cast<int64_t>(kt) * 16 + 2 * (lane & 3)) * pitch + n0 / 8;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const uint4* row = reinterpret_cast<const uint4*>(src + ((r & 1) + 8 * (r >> 1)) * pitch);
-      w[2 * r] = __ldg(row);
-      w[2 * r + 1] = __ldg(row + 1);
-    }
-  }
-  __device__ __forceinline__ void Store(uint32_t* out, int lane) const {
-    const int g = lane >> 2;
-    const int shift = 4 * ((g >> 1) + 4 * (g & 1));
-    uint32_t m[4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      uint32_t v[4][2];  // rows 2c, 2c + 1, 2c + 8, 2c + 9; columns g, g + 8
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint4& q = w[2 * r + (t >> 1)];
-        v[r][0] = ((t & 1) ? q.z : q.x) >> shift;
-        v[r][1] = ((t & 1) ? q.w : q.y) >> shift;
-      }
-      m[t] = (v[0][0] & 0xFu) | ((v[2][0] & 0xFu) << 4) | ((v[0][1] & 0xFu) << 8) | ((v[2][1] & 0xFu) << 12) |
-             ((v[1][0] & 0xFu) << 16) | ((v[3][0] & 0xFu) << 20) | ((v[1][1] & 0xFu) << 24) | (v[3][1] << 28);
-    }
-    reinterpret_cast<uint4*>(out)[lane] = make_uint4(m[0], m[1], m[2], m[3]);
   }
 };
 
@@ -351,11 +321,8 @@ extern "C" int infiniops_b200_awq_marlin_repack(const int32_t* b_q_weight, int64
   if (const int rc = CheckCommon(b_q_weight, out, size_k, size_n, num_bits, is_a_8bit)) return rc;
   auto s = static_cast<cudaStream_t>(stream);
   if (num_bits == 4) {
-    if (is_a_8bit) return Launch<4, true, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
-    // (the warp kernel reads AWQ rows by 16-byte loads; `b_q_weight` itself may sit on any word)
-    return reinterpret_cast<uintptr_t>(b_q_weight) % 16 == 0
-               ? LaunchWarps<4, Source::kAwq>(b_q_weight, out, size_k, size_n, s)
-               : Launch<4, false, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
+    return is_a_8bit ? Launch<4, true, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s)
+                     : Launch<4, false, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s);
   }
   return is_a_8bit ? Launch<8, true, Source::kAwq>(b_q_weight, nullptr, out, size_k, size_n, s)
                    : LaunchWarps<8, Source::kAwq>(b_q_weight, out, size_k, size_n, s);
