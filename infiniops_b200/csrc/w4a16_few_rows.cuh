@@ -24,7 +24,7 @@ struct FewRowsParams {
   const int32_t* expert_ids;
   const int32_t* num_post_pad;
   const float* topk_weights;
-  int top_k, block_size, mul_weights, out_rows, a_sorted, out_sorted, blocks;
+  int top_k, block_size, mul_weights, out_rows, a_sorted, out_sorted, blocks, experts;
   int fuse_silu;           // columns are gate and up interleaved in runs of 16; stores silu(gate) * up, [rows][N/2]
 };
 

@@ -2883,6 +2883,7 @@ extern "C" int infiniops_b200_moe_wna16_marlin_gemm_ex(
     f.a_sorted = a_sorted || gathers ? 1 : 0;
     f.out_sorted = p.out_sorted;
     f.blocks = static_cast<int>(blocks);
+    f.experts = static_cast<int>(num_experts);
     f.fuse_silu = p.fuse_silu;
     return FewRowsGemm(a_dtype, FewRowsWeightsOf(b_type_id), f, s);
   }
