@@ -2754,9 +2754,16 @@ extern "C" int infiniops_b200_moe_wna16_marlin_gemm_ex(
   const int gather_grid = static_cast<int>(std::min<int64_t>(sorted_cap, 4 * NumSms()));
   // Routing blocks of up to 16 rows: the register-operand kernel, which reads the tokens' rows where they are
   // unless the gather has something else to do (column order, by-products); no scatter, no completion signal.
-  // One token over 8 experts of 4096 / 14336: 109 -> 94 us for the whole chain; 16 tokens over 256 of 7168 / 2048,
-  // top 8: 820 -> 787 us.
-  const bool few_rows = moe_block_size <= kFewRows && (options == nullptr || (options->row_dest == nullptr && options->signal == nullptr)) &&
+  // Where the line lies (time against the tensor-memory kernel's with its gather, cold, even routing):
+  //  * 8-row blocks, 0.25 to 128 rows per expert: 0.6 to 0.92 in every shape measured.
+  //  * 16-row blocks of 8-bit weights: at most 0.76, full blocks included.
+  //  * 16-row blocks of 4-bit weights: uint4 0.75 to 1.04 up to 32 rows per expert (1.07 to 1.13, with rows already
+  //    sorted, at two shapes of K = 14336), 1.00 to 1.10 from 64 on: its zero points cost registers; uint4b8 0.78 to
+  //    1.01 up to 64, 0.93 to 1.02 at 128, up to 1.04 at 512.
+  // (Rows that all go to an eighth of the experts: up to 1.13 at 16-row blocks; the host cannot know.)
+  const int64_t most_rows = moe_block_size == 8 || BitsOf(b_type_id) == 8 ? INT32_MAX : b_zeros != nullptr ? 32 : 128;
+  const bool few_rows = moe_block_size <= kFewRows && size_m * top_k / num_experts <= most_rows &&
+                        (options == nullptr || (options->row_dest == nullptr && options->signal == nullptr)) &&
                         blocks * (size_n / 64) <= (1 << 24);
   const bool gathers = perm != nullptr || (!a_sorted && !(few_rows && position == nullptr && block_rows_out == nullptr));
   if (position != nullptr &&
