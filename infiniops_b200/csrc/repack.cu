@@ -132,7 +132,8 @@ RepackKernel(const uint32_t* __restrict__ in, const int32_t* __restrict__ perm,
 // 80.6 -> 46.8, AWQ 8-bit 77.1 -> 64.2; 4096 x 4096 9.2 -> 5.4, 14.6 -> 9.5, 14.1 -> 11.9.  Not for 4-bit AWQ, whose
 // words hold eight columns of a row: eight lanes then load the same words for one nibble of each, 55.9 us staged
 // and 57.9 this way (2.6 and 3.5 at 1024 x 1024).
-constexpr int kUnroll = 4;
+template <int kBits, Source kSource>
+constexpr int kTilesPerWarp = kBits == 4 ? 4 : kSource == Source::kGptq ? 2 : 1;
 
 // x = four bytes (one per source) -> low nibbles in bits 0..15, high nibbles in bits 16..31.
 __device__ __forceinline__ uint32_t SplitNibbles(uint32_t x) {
@@ -237,7 +238,7 @@ struct WarpTile<8, Source::kAwq> {
 template <int kBits, Source kSource>
 __global__ void __launch_bounds__(kThreads) RepackWarpKernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                             int size_k, int size_n) {
-  constexpr int kU = kBits == 8 && kSource == Source::kAwq ? 1 : kBits == 8 || kSource == Source::kAwq ? 2 : kUnroll;
+  constexpr int kU = kTilesPerWarp<kBits, kSource>;
   const int lane = threadIdx.x & 31, chunks = size_n / 64, tiles = size_k / 16;
   const long long unit = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
   const int kt0 = static_cast<int>(unit / chunks) * kU, chunk = static_cast<int>(unit % chunks);
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(kThreads) RepackWarpKernel(const uint32_t* __r
 
 template <int kBits, Source kSource>
 int LaunchWarps(const int32_t* in, int32_t* out, int64_t size_k, int64_t size_n, cudaStream_t stream) {
-  constexpr int kU = kBits == 8 && kSource == Source::kAwq ? 1 : kBits == 8 || kSource == Source::kAwq ? 2 : kUnroll;
+  constexpr int kU = kTilesPerWarp<kBits, kSource>;
   const int64_t units = (size_n / 64) * ((size_k / 16 + kU - 1) / kU);
   const int64_t blocks = (units + kThreads / 32 - 1) / (kThreads / 32);
   RepackWarpKernel<kBits, kSource><<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(
@@ -307,8 +308,11 @@ extern "C" int infiniops_b200_gptq_marlin_repack(const int32_t* b_q_weight, cons
                          : Launch<8, false, Source::kGptqPerm>(b_q_weight, perm, out, size_k, size_n, s);
   }
   if (num_bits == 4) {
-    return is_a_8bit ? Launch<4, true, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s)
-                     : LaunchWarps<4, Source::kGptq>(b_q_weight, out, size_k, size_n, s);
+    if (is_a_8bit) return Launch<4, true, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s);
+    // Small matrices leave the warp form too few warps: 2.6 us staged and 2.8 us this way at 1024 x 1024, 2.7 and 2.9 at
+    // 1536 x 1024, but 3.3 and 3.0 at 1024 x 3072.
+    return size_k * size_n < (2 << 20) ? Launch<4, false, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s)
+                                       : LaunchWarps<4, Source::kGptq>(b_q_weight, out, size_k, size_n, s);
   }
   return is_a_8bit ? Launch<8, true, Source::kGptq>(b_q_weight, nullptr, out, size_k, size_n, s)
                    : LaunchWarps<8, Source::kGptq>(b_q_weight, out, size_k, size_n, s);

@@ -1,5 +1,6 @@
 """GPU: the warp-per-chunk repack at the edges of its work split (a single k-tile, tile counts that do not divide
-by the tiles a warp takes, one and three 64-column chunks), every source and width, bit for bit."""
+by the tiles a warp takes, one and three 64-column chunks), every source and width, bit for bit.  4-bit AWQ and
+small 4-bit GPTQ matrices take the staged form."""
 
 import numpy as np
 import pytest
@@ -10,7 +11,7 @@ from oracle import quant as oq
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("k,n", ((16, 64), (80, 192), (1040, 64)))
+@pytest.mark.parametrize("k,n", ((16, 64), (80, 192), (1040, 64), (1040, 2112)))   # (the last: GPTQ 4-bit, from 2 Mi weights on)
 @pytest.mark.parametrize("bits", (4, 8))
 @pytest.mark.parametrize("source", ("gptq", "awq"))
 def test_repack_edges(source, bits, k, n):
