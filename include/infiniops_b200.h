@@ -336,7 +336,10 @@ typedef struct {
 } iob_peer_signal;
 
 /* infiniops_b200_marlin_gemm for a problem given as a struct, with output placement, peer outputs
- * and an optional completion signal (NULL = none).  No counterpart in the reference. */
+ * and an optional completion signal (NULL = none).  Up to 16 rows the kernel depends on them: without
+ * peers and signal the register-operand kernel, with either the tensor-memory kernel, whose fp32 sums
+ * come in another order -- the two may round a result to neighbouring values.  No counterpart in
+ * the reference. */
 int infiniops_b200_marlin_gemm_placed(const iob_gemm_problem* problem, int a_dtype,
                                       int64_t b_type_id, const iob_peer_signal* signal,
                                       void* scratch, size_t scratch_bytes, void* stream);
@@ -350,9 +353,10 @@ size_t infiniops_b200_marlin_gemm_batch_scratch_bytes(void);
  * problems per launch at most).  Inside a launch the (tile, k-stage) units of all problems form
  * one sequence cut into equal ranges, one per thread block, so pipelines never drain between
  * problems and launch, set-up and tail are paid once per launch instead of once per GEMM.
- * Results are identical to calling infiniops_b200_marlin_gemm per problem up to the order of the
- * fp32 split-K additions (deterministic for a given problem list).  `signal` (or NULL) rides on
- * the last launch.  Same scratch rules as infiniops_b200_marlin_gemm.
+ * Results are deterministic for a given problem list, and those of infiniops_b200_marlin_gemm per
+ * problem up to the order of the fp32 additions: problems of up to 16 rows run another kernel there
+ * (see infiniops_b200_marlin_gemm_placed), larger ones split K in other places, so a result may round
+ * to the neighbouring value.  `signal` (or NULL) rides on the last launch.  Same scratch rules as infiniops_b200_marlin_gemm.
  * No counterpart in the reference. */
 int infiniops_b200_marlin_gemm_batch(const iob_gemm_problem* problems, int count, int a_dtype,
                                      int64_t b_type_id, const iob_peer_signal* signal,

@@ -135,6 +135,16 @@ def _worker(rank, world, port):
         g = capi.gemm_problem(a, marlin, None, s, z, full_out, m, n // world, k, out_ld=n, out_col0=rank * (n // world),
                               peer_out=[group.address(r, off) for r in group.others()])
         scratch = torch.zeros(capi.lib().infiniops_b200_marlin_gemm_batch_scratch_bytes(), dtype=torch.uint8, device=dev)
+        # What the batched call computes for this shard alone, all-gathered.  It runs the tensor-memory kernel, while
+        # up to 16 rows `marlin_gemm` runs another one: the same fp32 sums in another order, so the two may round to
+        # neighbouring values (half an ulp each, 2^-8, and the sums' own 1.5e-4), not further apart.
+        alone = torch.empty((m, n // world), dtype=torch.bfloat16, device=dev)
+        capi.marlin_gemm_batch(capi.problem_array([capi.gemm_problem(a, marlin, None, s, z, alone, m, n // world, k)]),
+                               torch.bfloat16, capi.QTYPE_UINT4, scratch)
+        batched = parallel.as_matrix(parallel.gather_columns(alone))
+        torch.cuda.synchronize()
+        err5 = float((batched.float() - sharded.float()).abs().max() / sharded.float().abs().max())
+        assert err5 <= 2.0 ** -7 + 3e-4, err5
         for _ in range(2):
             capi.marlin_gemm_batch(capi.problem_array([g]), torch.bfloat16, capi.QTYPE_UINT4, scratch,
                                    signal=group.signal())
@@ -142,7 +152,7 @@ def _worker(rank, world, port):
             torch.cuda.synchronize()
             assert group.wait_status() == (0, 0) and capi.scratch_status(scratch) == 0
             # each rank's slice equals what the all-gather formulation delivered
-            assert torch.equal(full_out, sharded)
+            assert torch.equal(full_out, batched)
             dist.barrier()
         # the same again with the slices sent by one copy launch behind the GEMM (local placement only)
         full_out.zero_()
@@ -158,7 +168,7 @@ def _worker(rank, world, port):
             group.wait()
             torch.cuda.synchronize()
             assert group.wait_status() == (0, 0) and capi.scratch_status(scratch) == 0
-            assert torch.equal(full_out, sharded)
+            assert torch.equal(full_out, batched)
             dist.barrier()
         group.close()
     finally:

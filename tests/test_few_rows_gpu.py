@@ -43,11 +43,12 @@ def _qtype(bits, zeros):
     (8, 640, 192, 64),      # five chunks, two groups in each
     (9, 1152, 64, 128),     # nine chunks: the first row of the second token tile
     (16, 2560, 320, -1),    # twenty chunks over a cluster, one group
-    (5, 2304, 9536, 256),   # a tile more than one round of blocks
+    (5, 2304, None, 256),   # a tile more than one round of blocks (two per SM): the others whole, that one over a cluster
 ))
 def test_dense_edges(m, k, n, group, bits, zeros, dtype):
     from infiniops_b200 import capi
 
+    n = n or 64 * (2 * torch.cuda.get_device_properties(0).multi_processor_count + 1)
     (q, scales, z), (w, s, zd) = _weights(bits, k, n, group, dtype, zeros, m + k)
     gen = torch.Generator().manual_seed(m)
     a, bias = torch.randn((m, k), generator=gen).to(dtype), torch.randn(n, generator=gen).to(dtype)
@@ -58,15 +59,40 @@ def test_dense_edges(m, k, n, group, bits, zeros, dtype):
     assert rel_max_err(out[:m], oq.w4a16_gemm(a, q, scales, z, bits, bias=bias)) <= TOL[dtype]
 
 
-@pytest.mark.parametrize("block", (8, 16))
-@pytest.mark.parametrize("by_product", (False, True))   # rows read where they are / through the gather
-@pytest.mark.parametrize("tokens,experts,k,n,bits", ((1, 8, 512, 128, 4), (11, 4, 1152, 192, 8), (70, 3, 256, 64, 4)))
-def test_routed_edges(tokens, experts, k, n, bits, by_product, block):
+@pytest.mark.parametrize("m", (1, 9, 16))
+def test_placed_without_peers(m):
+    """Columns [n, 2n) of a 3n-wide matrix: the bits of the plain call, nothing beside them -- and the batched call's
+    result, which another kernel computes, to the rounding of each."""
     from infiniops_b200 import capi
 
-    top_k, dtype = 2, torch.bfloat16
-    hosts, devs = zip(*[_weights(bits, k, n, 128, dtype, True, 50 + e) for e in range(experts)])
-    w, s, z = (torch.stack(x) for x in zip(*devs))
+    k, n, dtype = 1152, 192, torch.bfloat16
+    _, (w, s, z) = _weights(4, k, n, 128, dtype, True, 60 + m)
+    a = torch.randn((m, k), generator=torch.Generator().manual_seed(m)).to(dtype).cuda()
+    plain, batched = (torch.empty((m, n), dtype=dtype, device="cuda") for _ in range(2))
+    capi.marlin_gemm(a, w, None, s, z, capi.QTYPE_UINT4, m, n, k, plain)
+    wide = torch.full((m, 3 * n), 7.0, dtype=dtype, device="cuda")
+    scratch = torch.zeros(max(capi.lib().infiniops_b200_marlin_gemm_scratch_bytes(m, n, k),
+                              capi.lib().infiniops_b200_marlin_gemm_batch_scratch_bytes()), dtype=torch.uint8, device="cuda")
+    capi.marlin_gemm_placed(capi.gemm_problem(a, w, None, s, z, wide, m, n, k, out_ld=3 * n, out_col0=n), dtype,
+                            capi.QTYPE_UINT4, scratch)
+    capi.marlin_gemm_batch(capi.problem_array([capi.gemm_problem(a, w, None, s, z, batched, m, n, k)]), dtype,
+                           capi.QTYPE_UINT4, scratch)
+    torch.cuda.synchronize()
+    assert torch.equal(wide[:, n:2 * n], plain)
+    assert bool((wide[:, :n] == 7.0).all()) and bool((wide[:, 2 * n:] == 7.0).all())
+    assert rel_max_err(batched, plain) <= 2 * TOL[dtype]
+
+
+@pytest.mark.parametrize("block", (8, 16))
+@pytest.mark.parametrize("dtype,group,zeros", ((torch.bfloat16, 128, True), (torch.float16, 64, False)))
+@pytest.mark.parametrize("by_product", (False, True))   # rows read where they are / through the gather
+@pytest.mark.parametrize("tokens,experts,k,n,bits", ((1, 8, 512, 128, 4), (11, 4, 1152, 192, 8), (40, 3, 256, 64, 4), (70, 3, 256, 64, 4)))
+def test_routed_edges(tokens, experts, k, n, bits, by_product, dtype, group, zeros, block):
+    from infiniops_b200 import capi
+
+    top_k = 2
+    hosts, devs = zip(*[_weights(bits, k, n, group, dtype, zeros, 50 + e) for e in range(experts)])
+    w, s, z = (torch.stack(x) if x[0] is not None else None for x in zip(*devs))
     gen = torch.Generator().manual_seed(tokens)
     ids = torch.randint(0, experts, (tokens, top_k), generator=gen, dtype=torch.int32)
     x = torch.randn((tokens, k), generator=gen).to(dtype)
@@ -81,9 +107,9 @@ def test_routed_edges(tokens, experts, k, n, bits, by_product, block):
     extra = {"block_rows": torch.empty(blocks + 1, dtype=torch.int32, device="cuda")} if by_product else {}
     args = (x.cuda(), w, bias.cuda(), s, z, sorted_ids, expert_ids, npost, tw.cuda(), block, top_k)
     out = torch.full((rows, n), float("nan"), dtype=dtype, device="cuda")
-    capi.moe_wna16_marlin_gemm(*args, True, _qtype(bits, True), tokens, n, k, out, **extra)
+    capi.moe_wna16_marlin_gemm(*args, True, _qtype(bits, zeros), tokens, n, k, out, **extra)
     in_order = torch.full((size, n), float("nan"), dtype=dtype, device="cuda")
-    capi.moe_wna16_marlin_gemm(*args, False, _qtype(bits, True), tokens, n, k, in_order, out_sorted=True, **extra)
+    capi.moe_wna16_marlin_gemm(*args, False, _qtype(bits, zeros), tokens, n, k, in_order, out_sorted=True, **extra)
     torch.cuda.synchronize()
     ref = torch.cat([oq.w4a16_gemm(x[r // top_k:r // top_k + 1], *hosts[int(ids.view(-1)[r])], bits,
                                    bias=bias[int(ids.view(-1)[r])]) for r in range(rows)])
