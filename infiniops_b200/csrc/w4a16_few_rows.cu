@@ -13,16 +13,22 @@
 // Split: a warp owns 64 columns and every kWarps-th 128-k chunk of its block's share of K; kWarps warps are a
 // block, up to eight blocks that share a column tile are a cluster.  Partial sums meet in shared memory and
 // over the cluster's distributed shared memory in a fixed order: no scratch, no counters, the same bits on
-// every run.  Each warp keeps 4 KB of weights in flight ahead of their use, refilled slab by slab.
+// every run.  Each warp keeps 4 KB of weights in flight ahead of their use (8 KB of 8-bit weights at up to 8 rows),
+// refilled slab by slab.
 // Activations of a chunk (live rows only) and its scales and zero points come the same way into a warp's own
 // double buffer, so no block-wide barrier stands in the main loop.
 //
 // Scales are applied per group in fp32 to the products of the exact integers.
 //
+// Two token tiles of 4-bit weights sit at the cap of 128 registers (two blocks an SM) and spill 16 to 24 bytes, as do two
+// tiles of 8-bit weights with zero points in bfloat16.
+//
 // Measured, cold L2, against the tensor-memory kernel: the four linears of a 4096 / 14336 layer as four launches,
-// 74.9 -> 68.5 us at 1 row (uint4), 73.5 -> 61.7 at 16 rows (uint4b8, float16), 121.5 -> 64.3 at 7 rows (8-bit,
-// 3.5 TB/s).  Not for a batch of linears in one launch: the persistent blocks of the tensor-memory kernel pay their
+// 74.9 -> 67.5 us at 1 row (uint4), 73.6 -> 61.8 at 16 rows (uint4b8, float16), 121.6 -> 66.6 at 7 rows (8-bit,
+// 3.4 TB/s).  Not for a batch of linears in one launch: the persistent blocks of the tensor-memory kernel pay their
 // set-up once for all of them (sixteen linears of 1..64 rows: 191 us, with the small ones here 200).
+// Error against 64-bit arithmetic: the rounding of the result (0.00165 in the 2-norm for bfloat16), where the other
+// kernel also rounds the scaled weights of 8-bit types and groups of 64 (0.0023).
 #include "w4a16_few_rows.cuh"
 
 #include <algorithm>
@@ -244,7 +250,7 @@ __device__ __forceinline__ void FewRowsTile(const FewRowsParams& p, int tile, in
   };
   if constexpr (!kMoe) {
     // Nothing that a predecessor in the stream could have written is read before the wait: not the activations, and
-    // not the weights, after a repack or an update.  (Weight copies ahead of it would give 0.2 to 1 us a launch:
+    // not the weights, after a repack or an update.  (Weight copies ahead of it would give 0.2 to 1.7 us a launch:
     // 4096 x 28672, 1 row, back to back 20.3 us against 21.2 with 4-bit weights, 26.8 against 28.5 with 8-bit ones.
     // Pulling the slabs into L2 instead gives nothing: 21.2 to 21.5 us and 28.9 to 29.3.)
     set_rows();

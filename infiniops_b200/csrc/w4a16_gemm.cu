@@ -2561,8 +2561,10 @@ extern "C" int infiniops_b200_marlin_gemm_placed(const iob_gemm_problem* problem
     activations = base + plan.gathered_off;
   }
   // Up to 16 rows: the register-operand kernel (no peers to write, no completion signal to give).  The four
-  // linears of a 4096 / 14336 layer, a launch each: 74.9 -> 68.5 us at 1 row (uint4), 73.5 -> 61.7 at 16
-  // (uint4b8, float16), 121.5 -> 64.3 at 7 (8-bit).  The line lies at its second token tile of 8.
+  // linears of a 4096 / 14336 layer, a launch each: 74.9 -> 67.5 us at 1 row (uint4), 73.6 -> 61.8 at 16
+  // (uint4b8, float16), 121.6 -> 66.6 at 7 (8-bit).  16 rows is the most that kernel takes; it is no slower there in any
+  // of nine shapes from 1024 x 1536 to 14336 x 4096 and five weight types (0.31 to 1.00 of the time, the last at
+  // 4096 x 28672 with 16 rows of uint4).
   if (g.size_m <= kFewRows && g.n_peers == 0 && signal == nullptr) {
     return FewRowsGemm(a_dtype, FewRowsWeightsOf(b_type_id), FewRowsOf(g, p, activations), static_cast<cudaStream_t>(stream));
   }
